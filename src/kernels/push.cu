@@ -37,6 +37,7 @@
 #include "common/cuda.h"
 #include "common/trace.h"
 #include "kernels/run_copy.cuh"
+#include "kernels/smem_limit.h"
 
 #include <algorithm>
 #include <atomic>
@@ -1720,6 +1721,12 @@ void launchMaybeDependent(Kernel kernel, uint32_t grid, uint32_t threads, size_t
   cudaLaunchKernelEx(&cfg, kernel, p);
 }
 
+template <typename Kernel>
+void allowSmem(Kernel kernel, size_t bytes) {
+  check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)),
+        "cudaFuncSetAttribute");
+}
+
 template <int N>
 void launchOne(const PushEntry* entries, uint32_t n, uint32_t bulkTiles, uint32_t plainTiles, uint32_t blockTiles,
                uint32_t bulkTileBytes, uint32_t bulkStages, cudaStream_t stream, int maxCtas, uint32_t* flag, uint32_t flagValue,
@@ -1766,13 +1773,8 @@ void launchOne(const PushEntry* entries, uint32_t n, uint32_t bulkTiles, uint32_
     if (grid == 0) grid = 1;
     size_t lightSmem = static_cast<size_t>(kWarps) * p.warpTileBytes;
     if (blockTiles > 0) lightSmem = std::max<size_t>(lightSmem, kBlockStagesLight * (kBlockTileBytes + sizeof(uint64_t)));
-    static size_t lightConfigured[64] = {};
-    if (lightSmem > 48 * 1024 && dev < 64 && lightConfigured[dev] < lightSmem) {
-      check(cudaFuncSetAttribute(tpb_push_pack_light<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(lightSmem)),
-            "cudaFuncSetAttribute");
-      lightConfigured[dev] = lightSmem;
-    }
+    static SmemLimit lightLimit;
+    if (lightSmem > 48 * 1024) lightLimit.raise(dev, lightSmem, [](size_t most) { allowSmem(tpb_push_pack_light<N>, most); });
     launchMaybeDependent(tpb_push_pack_light<N>, grid, kLightThreads, lightSmem, stream, p, dependent);
     check(cudaGetLastError(), "tpb_push_pack_light launch");
     ++gLaunches;
@@ -1781,12 +1783,8 @@ void launchOne(const PushEntry* entries, uint32_t n, uint32_t bulkTiles, uint32_
   const size_t smem = static_cast<size_t>(bulkStages) * bulkTileBytes + (kThreads / 32 - 1) * p.warpTileBytes +
       kMaxBulkStages * sizeof(uint64_t) + 128;
   if (smem > kMaxSmemPerCta) throw std::runtime_error("push plan needs more shared memory than a CTA has");
-  static size_t configured[64] = {};
-  if (dev < 64 && configured[dev] < smem) {
-    check(cudaFuncSetAttribute(tpb_push_pack<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
-          "cudaFuncSetAttribute");
-    configured[dev] = smem;
-  }
+  static SmemLimit limit;
+  limit.raise(dev, smem, [](size_t most) { allowSmem(tpb_push_pack<N>, most); });
   constexpr uint32_t kPlainWarps = kThreads / 32 - 1;
   uint32_t want = bulkTiles;
   const uint32_t plainCtas = (plainTiles + kPlainWarps - 1) / kPlainWarps;
