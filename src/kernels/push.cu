@@ -36,6 +36,7 @@
 
 #include "common/cuda.h"
 #include "common/trace.h"
+#include "kernels/block_pipe.h"
 #include "kernels/run_copy.cuh"
 #include "kernels/smem_limit.h"
 
@@ -1085,6 +1086,21 @@ constexpr uint32_t kBlockStagesLight = 3;  // 102 KiB: two CTAs on an SM
 static_assert(kBlockTileBytes + 64 <= 8 * kWideWarpTileBytes, "one tile fits the eight warps' own staging areas");
 
 __device__ __forceinline__ void blockBarrier() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+// The same barrier; tells whether any of the threads came with `bad`.
+__device__ __forceinline__ bool blockBarrierAny(bool bad) {
+  uint32_t any;
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.u32 p, %1, 0;\n"
+      "bar.red.or.pred q, 1, 256, p;\n"
+      "selp.u32 %0, 1, 0, q;\n"
+      "}\n"
+      : "=r"(any)
+      : "r"(static_cast<uint32_t>(bad))
+      : "memory");
+  return any != 0;
+}
 
 template <typename S, typename D, bool kConvert>
 __device__ __forceinline__ D convertOne(S v) {
@@ -1105,9 +1121,7 @@ __device__ __forceinline__ uint32_t packPair(D lo, D hi) {
 struct BlockPipe {
   uint8_t* buffers;
   uint64_t* full;  // one barrier per stage, kBlockSlots arrivals each
-  uint32_t stages;
-  uint32_t issued, taken;
-  bool failed;
+  TileRing ring;
 };
 
 template <typename S, typename D, bool kConvert, bool kNarrow>
@@ -1153,10 +1167,9 @@ struct BlockTransposer {
   }
 
   // One copy per thread of the first kBlockSlots. Every one of them arrives, with the bytes it sends for.
-  __device__ __forceinline__ void issue(uint32_t t) {
-    const uint32_t stage = pipe.issued % pipe.stages;
-    ++pipe.issued;
+  __device__ __forceinline__ void issue(uint32_t t, uint32_t stage) {
     if (tid >= kBlockSlots) return;
+    fenceProxyAsync();  // the stage may have been read until the barrier before this
     const Place p = place(t);
     const int left = p.nr - static_cast<int>(myChunk) * kRows, nr = left < kRows ? left : kRows;
     uint32_t bytes = 0;
@@ -1322,29 +1335,17 @@ struct BlockTransposer {
     }
   }
 
-  __device__ __forceinline__ void run(uint32_t first, uint32_t step) {
-    uint32_t ahead = first;  // next tile to send for
-    for (uint32_t s = 0; s < pipe.stages && ahead < a.numTiles; ++s, ahead += step) issue(ahead);
-#pragma unroll 1
-    for (uint32_t t = first; t < a.numTiles; t += step) {
-      const uint32_t stage = pipe.taken % pipe.stages;
-      // A copy that never completes: what is left is not written, and the launch reports it.
-      if (!pipe.failed) pipe.failed = !mbarWaitBounded(&pipe.full[stage], (pipe.taken / pipe.stages) & 1);
-      ++pipe.taken;
-      const uint8_t* buffer = pipe.buffers + stage * kBlockTileBytes;
-      if (!pipe.failed) {
-        const Place p = place(t);
-        if constexpr (kNarrow) writeRun(buffer, p);
-        else if (p.nr == kRows && p.nc == kBlockSlots) writeRows<true>(buffer, p);
-        else writeRows<false>(buffer, p);
-      }
-      blockBarrier();  // everybody is through with this stage
-      if (ahead < a.numTiles) {
-        fenceProxyAsync();
-        issue(ahead);
-        ahead += step;
-      }
-    }
+  // A warp whose lanes do not all see the tile writes none of it: rows are put together across the lanes.
+  __device__ __forceinline__ bool arrived(uint32_t stage, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbarWaitBounded(&pipe.full[stage], parity)) != 0;
+  }
+  __device__ __forceinline__ bool anyone(bool bad) { return blockBarrierAny(bad); }
+  __device__ __forceinline__ void take(uint32_t t, uint32_t stage) {
+    const uint8_t* buffer = pipe.buffers + stage * kBlockTileBytes;
+    const Place p = place(t);
+    if constexpr (kNarrow) writeRun(buffer, p);
+    else if (p.nr == kRows && p.nc == kBlockSlots) writeRows<true>(buffer, p);
+    else writeRows<false>(buffer, p);
   }
 };
 
@@ -1352,8 +1353,9 @@ template <typename S, typename D, bool kConvert, bool kNarrow>
 __device__ __noinline__ void blockTilesOfForm(const PushEntry& e, uint32_t first, uint32_t step, int tid, BlockPipe& pipe) {
   const StridedArgs a = loadStridedArgs(e);
   BlockPipe mine = pipe;
-  BlockTransposer<S, D, kConvert, kNarrow>(a, mine, tid).run(first, step);
-  pipe = mine;
+  BlockTransposer<S, D, kConvert, kNarrow> transposer(a, mine, tid);
+  takeTiles(mine.ring, a.numTiles, first, step, transposer);
+  pipe.ring = mine.ring;
 }
 template <typename S, typename D, bool kConvert>
 __device__ __forceinline__ void blockTilesTyped(const PushEntry& e, uint32_t first, uint32_t step, int tid, BlockPipe& pipe) {
@@ -1361,20 +1363,21 @@ __device__ __forceinline__ void blockTilesTyped(const PushEntry& e, uint32_t fir
   else blockTilesOfForm<S, D, kConvert, false>(e, first, step, tid, pipe);
 }
 
-// Block tiles first, first + step, ... of the block class; the kBlockThreads threads of `tid` take part. False
-// if a copy never completed.
+// Block tiles first, first + step, ... of the block class; the kBlockThreads threads of `tid` take part. False,
+// for all of them alike, if a copy never completed: what is left is not written, the launch reports it, and the memory
+// of the stages is not to be used again.
 template <int N>
 __device__ __forceinline__ bool runBlockTiles(const PushParams<N>& p, uint32_t first, uint32_t step, int tid, uint8_t* mem) {
   constexpr uint32_t F32 = static_cast<uint32_t>(DType::kF32), BF = static_cast<uint32_t>(DType::kBF16),
                      F16 = static_cast<uint32_t>(DType::kF16);
-  BlockPipe pipe{mem, reinterpret_cast<uint64_t*>(mem + p.blockStages * kBlockTileBytes), p.blockStages, 0, 0, false};
+  BlockPipe pipe{mem, reinterpret_cast<uint64_t*>(mem + p.blockStages * kBlockTileBytes), TileRing{p.blockStages, 0, 0, false}};
   if (tid == 0) {
     for (uint32_t s = 0; s < p.blockStages; ++s) mbarInit(&pipe.full[s], kBlockSlots);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   blockBarrier();
   uint32_t t = first;
-  while (t < p.blockTiles) {
+  while (t < p.blockTiles && !pipe.ring.failed) {
     const PushEntry& e = *findEntry(p, t, kBlockClass);
     const uint32_t local = t - e.tileStart;
     if (e.srcDtype == e.dstDtype) {
@@ -1396,12 +1399,20 @@ __device__ __forceinline__ bool runBlockTiles(const PushParams<N>& p, uint32_t f
     }
     t += (e.numTiles - local + step - 1) / step * step;
   }
-  if (pipe.failed) reportStatus(p.status, kStatusBarrierTimeout);
+  if (pipe.ring.failed) {
+    if (tid == 0) {
+      waitForCopiesUnderWay(pipe.ring.taken, pipe.ring.issued, pipe.ring.stages,
+                            [&](uint32_t stage, uint32_t parity) { mbarWaitBounded(&pipe.full[stage], parity); });
+      reportStatus(p.status, kStatusBarrierTimeout);
+    }
+    blockBarrier();
+    return false;
+  }
   // The memory goes back to the warps' own tiles, behind the copies that were written there.
   if (tid == 0)
     for (uint32_t s = 0; s < p.blockStages; ++s) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smemAddr(&pipe.full[s])) : "memory");
   blockBarrier();
-  return !pipe.failed;
+  return true;
 }
 
 // Warp tiles t = firstWarp, firstWarp + totalWarps, ... of the plain class.
@@ -1587,8 +1598,9 @@ __global__ void __launch_bounds__(kThreads, 1) tpb_push_pack(const __grid_consta
     const uint32_t warp = tid / 32 - 1;
     // Eight of these warps share the block tiles; the others go straight to the tiles a warp does alone.
     if (p.blockTiles > 0 && warp < kBlockThreads / 32) failed = !runBlockTiles(p, blockIdx.x, gridDim.x, tid - 32, warpTiles);
-    runPlainWarp(p, blockIdx.x * kPlainWarps + warp, gridDim.x * kPlainWarps, tid & 31,
-                 warpTiles + warp * p.warpTileBytes);
+    if (!failed)
+      runPlainWarp(p, blockIdx.x * kPlainWarps + warp, gridDim.x * kPlainWarps, tid & 31,
+                   warpTiles + warp * p.warpTileBytes);
   }
   publish(p, failed);
 }
@@ -1607,7 +1619,8 @@ __global__ void __launch_bounds__(kLightThreads, 2) tpb_push_pack_light(const __
   static_assert(kLightThreads == kBlockThreads, "the whole light CTA shares a block tile");
   bool failed = false;
   if (p.blockTiles > 0) failed = !runBlockTiles(p, blockIdx.x, gridDim.x, threadIdx.x, lightTiles);
-  runPlainWarp(p, blockIdx.x * kWarps + warp, gridDim.x * kWarps, threadIdx.x & 31, lightTiles + warp * p.warpTileBytes);
+  if (!failed)
+    runPlainWarp(p, blockIdx.x * kWarps + warp, gridDim.x * kWarps, threadIdx.x & 31, lightTiles + warp * p.warpTileBytes);
   publish(p, failed);
 }
 
