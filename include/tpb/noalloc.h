@@ -26,8 +26,8 @@
  *     TPB_NOALLOC_TOO_MANY (split them over several calls on the same stream).
  *   - Calls are safe back to back on ONE stream. Calls whose kernels could overlap on a GPU (different
  *     streams, or different threads launching at once) share the array of counters: serialise them.
- *   - The first call on each device looks up the array's device address (with that device current).
- *     Make that first call before starting any stream capture.
+ *   - The first call on each device looks up the array's device address and loads the kernels for tables of
+ *     every size (with that device current). Make that first call before starting any stream capture.
  *
  * Returns TPB_NOALLOC_OK (0) or a negative code; tpb_noalloc_strerror() explains a code.
  */

@@ -93,7 +93,7 @@ cudaError_t launch(const TableEntry* entries, uint32_t n, uint32_t tiles, uint32
 thread_local std::string t_lastCudaError;
 
 // Device address of g_scratch for the current device and that device's SM count; both resolved
-// once per device.
+// once per device, when the kernel is loaded there too.
 int lookupScratch(unsigned char** out, int* smCount) {
   static std::mutex mu;
   static unsigned char* perDevice[kMaxDevices] = {};
@@ -112,6 +112,18 @@ int lookupScratch(unsigned char** out, int* smCount) {
       t_lastCudaError = std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e);
       cudaGetLastError();
       return TPB_NOALLOC_CUDA_ERROR;
+    }
+    // Both forms of the kernel are loaded now. Where modules load lazily, the first launch of a form would load it,
+    // which may allocate and synchronise, and may happen inside a capture that began after the caller's first call.
+    for (const void* form : {reinterpret_cast<const void*>(&tpb_noalloc_push_kernel<kSmallTable>),
+                             reinterpret_cast<const void*>(&tpb_noalloc_push_kernel<TPB_NOALLOC_MAX_ITEMS>)}) {
+      cudaFuncAttributes attributes;
+      e = cudaFuncGetAttributes(&attributes, form);
+      if (e != cudaSuccess) {
+        t_lastCudaError = std::string("loading the kernel: ") + cudaGetErrorString(e);
+        cudaGetLastError();
+        return TPB_NOALLOC_CUDA_ERROR;
+      }
     }
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) {
