@@ -10,8 +10,6 @@
 #include <pybind11/pybind11.h>
 #include <pybind11/stl.h>
 
-#include <cctype>
-
 #include <tpb/tpb.h>
 
 #include "kernels/push.h"
@@ -142,8 +140,10 @@ bool parseTensorRecord(const std::string& raw, std::string* dtype, std::vector<i
   if (raw.compare(0, open.size(), open) != 0) return false;
   const size_t end = raw.find('"', open.size());
   if (end == std::string::npos || raw.compare(end, middle.size(), middle) != 0) return false;
-  for (size_t i = open.size(); i < end; ++i)
-    if (!std::isalnum(static_cast<unsigned char>(raw[i])) && raw[i] != '_') return false;
+  for (size_t i = open.size(); i < end; ++i) {
+    const char c = raw[i];  // not isalnum, whose answer depends on the locale: the name becomes a Python string
+    if (!((c >= '0' && c <= '9') || (c >= 'A' && c <= 'Z') || (c >= 'a' && c <= 'z') || c == '_')) return false;
+  }
   *dtype = raw.substr(open.size(), end - open.size());
   size_t at = end + middle.size();
   if (raw.compare(at, std::string::npos, "]}") == 0) return true;
