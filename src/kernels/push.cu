@@ -1418,8 +1418,11 @@ __device__ __forceinline__ bool runBlockTiles(const PushParams<N>& p, uint32_t f
   return true;
 }
 
+// What a kernel has code for: contiguous copies and conversions; 2-D views moved by single warps too; block tiles too.
+enum Forms : int { kContiguousForms = 0, kWarpForms = 1, kAllForms = 2 };
+
 // Warp tiles t = firstWarp, firstWarp + totalWarps, ... of the plain class.
-template <int N>
+template <int N, int kForms>
 __device__ __forceinline__ void runPlainWarp(const PushParams<N>& p, uint32_t firstWarp, uint32_t totalWarps, int lane,
                                              uint8_t* tileMem) {
   uint32_t t = firstWarp;
@@ -1427,13 +1430,17 @@ __device__ __forceinline__ void runPlainWarp(const PushParams<N>& p, uint32_t fi
     const PushEntry* e = findEntry(p, t, kPlainClass);
     const uint32_t local = t - e->tileStart;
     // One call handles every tile of this entry that falls to this warp.
-    if (e->kind == kCopyPlain) copyPlainTiles(*e, local, totalWarps, lane);
-    else if (e->kind == kCastPlain) castTiles(*e, local, totalWarps, lane);
-    else if (e->kind == kRows) rowTiles(*e, local, totalWarps, lane);
-    else if (e->kind == kStridedWide16) stridedWide16Tiles(*e, local, totalWarps, lane, tileMem);
-    else if (e->kind == kStridedNarrow) stridedNarrowTiles(*e, local, totalWarps, lane, tileMem);
-    else if (e->kind == kStridedBand) stridedBandTiles(*e, local, totalWarps, lane, tileMem);
-    else stridedTiles(*e, local, totalWarps, lane, tileMem);
+    if (e->kind == kCopyPlain) {
+      copyPlainTiles(*e, local, totalWarps, lane);
+    } else if (kForms == kContiguousForms || e->kind == kCastPlain) {
+      castTiles(*e, local, totalWarps, lane);
+    } else if constexpr (kForms != kContiguousForms) {
+      if (e->kind == kRows) rowTiles(*e, local, totalWarps, lane);
+      else if (e->kind == kStridedWide16) stridedWide16Tiles(*e, local, totalWarps, lane, tileMem);
+      else if (e->kind == kStridedNarrow) stridedNarrowTiles(*e, local, totalWarps, lane, tileMem);
+      else if (e->kind == kStridedBand) stridedBandTiles(*e, local, totalWarps, lane, tileMem);
+      else stridedTiles(*e, local, totalWarps, lane, tileMem);
+    }
     t += (e->numTiles - local + totalWarps - 1) / totalWarps * totalWarps;
   }
 }
@@ -1504,7 +1511,7 @@ __device__ __forceinline__ void publish(const PushParams<N>& p, bool failedHere)
 }
 
 // ---- the kernels --------------------------------------------------------------------------------
-template <int N>
+template <int N, int kForms>
 __global__ void __launch_bounds__(kThreads, 1) tpb_push_pack(const __grid_constant__ PushParams<N> p) {
   extern __shared__ uint8_t smemRaw[];
   // Layout: [bulk stages][warp tiles][mbarriers]; dynamic shared memory is only guaranteed to be
@@ -1600,15 +1607,17 @@ __global__ void __launch_bounds__(kThreads, 1) tpb_push_pack(const __grid_consta
     constexpr uint32_t kPlainWarps = kThreads / 32 - 1;
     const uint32_t warp = tid / 32 - 1;
     // Eight of these warps share the block tiles; the others go straight to the tiles a warp does alone.
-    if (p.blockTiles > 0 && warp < kBlockThreads / 32) failed = !runBlockTiles(p, blockIdx.x, gridDim.x, tid - 32, warpTiles);
+    if constexpr (kForms == kAllForms) {
+      if (p.blockTiles > 0 && warp < kBlockThreads / 32) failed = !runBlockTiles(p, blockIdx.x, gridDim.x, tid - 32, warpTiles);
+    }
     if (!failed)
-      runPlainWarp(p, blockIdx.x * kPlainWarps + warp, gridDim.x * kPlainWarps, tid & 31,
-                   warpTiles + warp * p.warpTileBytes);
+      runPlainWarp<N, kForms>(p, blockIdx.x * kPlainWarps + warp, gridDim.x * kPlainWarps, tid & 31,
+                              warpTiles + warp * p.warpTileBytes);
   }
   publish(p, failed);
 }
 
-template <int N>
+template <int N, int kForms>
 __global__ void __launch_bounds__(kLightThreads, 2) tpb_push_pack_light(const __grid_constant__ PushParams<N> p) {
   extern __shared__ __align__(16) uint8_t lightTiles[];  // kWarps * p.warpTileBytes, none for plain copies
   constexpr uint32_t kWarps = kLightThreads / 32;
@@ -1621,9 +1630,12 @@ __global__ void __launch_bounds__(kLightThreads, 2) tpb_push_pack_light(const __
   }
   static_assert(kLightThreads == kBlockThreads, "the whole light CTA shares a block tile");
   bool failed = false;
-  if (p.blockTiles > 0) failed = !runBlockTiles(p, blockIdx.x, gridDim.x, threadIdx.x, lightTiles);
+  if constexpr (kForms == kAllForms) {
+    if (p.blockTiles > 0) failed = !runBlockTiles(p, blockIdx.x, gridDim.x, threadIdx.x, lightTiles);
+  }
   if (!failed)
-    runPlainWarp(p, blockIdx.x * kWarps + warp, gridDim.x * kWarps, threadIdx.x & 31, lightTiles + warp * p.warpTileBytes);
+    runPlainWarp<N, kForms>(p, blockIdx.x * kWarps + warp, gridDim.x * kWarps, threadIdx.x & 31,
+                            lightTiles + warp * p.warpTileBytes);
   publish(p, failed);
 }
 
@@ -1743,8 +1755,8 @@ void allowSmem(Kernel kernel, size_t bytes) {
         "cudaFuncSetAttribute");
 }
 
-template <int N>
-void launchOne(const PushEntry* entries, uint32_t n, uint32_t bulkTiles, uint32_t plainTiles, uint32_t blockTiles,
+template <int N, int kForms>
+void launchForm(const PushEntry* entries, uint32_t n, uint32_t bulkTiles, uint32_t plainTiles, uint32_t blockTiles,
                uint32_t bulkTileBytes, uint32_t bulkStages, cudaStream_t stream, int maxCtas, uint32_t* flag, uint32_t flagValue,
                uint32_t* counter, uint32_t* status, const WaitBefore& wait, const DoneSlot& done, uint64_t bytesOut) {
   const bool publishes = flag != nullptr || wait.flag != nullptr || done.slot != nullptr;
@@ -1789,8 +1801,8 @@ void launchOne(const PushEntry* entries, uint32_t n, uint32_t bulkTiles, uint32_
     size_t lightSmem = static_cast<size_t>(kWarps) * p.warpTileBytes;
     if (blockTiles > 0) lightSmem = std::max<size_t>(lightSmem, kBlockStagesLight * (kBlockTileBytes + sizeof(uint64_t)));
     static SmemLimit lightLimit;
-    if (lightSmem > 48 * 1024) lightLimit.raise(dev, lightSmem, [](size_t most) { allowSmem(tpb_push_pack_light<N>, most); });
-    launchMaybeDependent(tpb_push_pack_light<N>, grid, kLightThreads, lightSmem, stream, p, dependent);
+    if (lightSmem > 48 * 1024) lightLimit.raise(dev, lightSmem, [](size_t most) { allowSmem(tpb_push_pack_light<N, kForms>, most); });
+    launchMaybeDependent(tpb_push_pack_light<N, kForms>, grid, kLightThreads, lightSmem, stream, p, dependent);
     check(cudaGetLastError(), "tpb_push_pack_light launch");
     ++gLaunches;
     return;
@@ -1799,7 +1811,7 @@ void launchOne(const PushEntry* entries, uint32_t n, uint32_t bulkTiles, uint32_
       kMaxBulkStages * sizeof(uint64_t) + 128;
   if (smem > kMaxSmemPerCta) throw std::runtime_error("push plan needs more shared memory than a CTA has");
   static SmemLimit limit;
-  limit.raise(dev, smem, [](size_t most) { allowSmem(tpb_push_pack<N>, most); });
+  limit.raise(dev, smem, [](size_t most) { allowSmem(tpb_push_pack<N, kForms>, most); });
   constexpr uint32_t kPlainWarps = kThreads / 32 - 1;
   uint32_t want = bulkTiles;
   const uint32_t plainCtas = (plainTiles + kPlainWarps - 1) / kPlainWarps;
@@ -1807,9 +1819,25 @@ void launchOne(const PushEntry* entries, uint32_t n, uint32_t bulkTiles, uint32_
   if (blockTiles > want) want = blockTiles;
   uint32_t grid = want < static_cast<uint32_t>(maxCtas) ? want : static_cast<uint32_t>(maxCtas);
   if (grid == 0) grid = 1;
-  launchMaybeDependent(tpb_push_pack<N>, grid, kThreads, smem, stream, p, dependent);
+  launchMaybeDependent(tpb_push_pack<N, kForms>, grid, kThreads, smem, stream, p, dependent);
   check(cudaGetLastError(), "tpb_push_pack launch");
   ++gLaunches;
+}
+
+// A message runs a kernel that has no code for forms it does not hold. Messages of one contiguous tensor are the
+// most frequent ones and mostly overhead, and what the forms of views keep across calls costs every launch of a
+// kernel that holds them. (Kernel times on one B200, everything in one kernel / this: 64 KiB copied 5.15 / 4.6 us, 1000
+// elements fp32 -> bf16 8.6 / 6.9; half a round trip of 4 KiB through a pipe 18.9 / 17.6.)
+template <int N, typename... Rest>
+void launchOne(const PushEntry* entries, uint32_t n, const Rest&... rest) {
+  int forms = kContiguousForms;
+  for (uint32_t i = 0; i < n; ++i) {
+    if (entries[i].kind == kTransposed) forms = kAllForms;
+    else if (isView(entries[i].kind) && forms == kContiguousForms) forms = kWarpForms;
+  }
+  if (forms == kAllForms) launchForm<N, kAllForms>(entries, n, rest...);
+  else if (forms == kWarpForms) launchForm<N, kWarpForms>(entries, n, rest...);
+  else launchForm<N, kContiguousForms>(entries, n, rest...);
 }
 
 }  // namespace

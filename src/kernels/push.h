@@ -47,6 +47,8 @@ constexpr inline TileClass tileClassOf(uint32_t kind) {
   return kind == kCopyBulk ? kBulkClass : kind == kTransposed ? kBlockClass : kPlainClass;
 }
 
+constexpr inline bool isView(uint32_t kind) { return kind != kCopyBulk && kind != kCopyPlain && kind != kCastPlain; }
+
 struct alignas(16) PushEntry {
   const void* src;
   void* dst;
