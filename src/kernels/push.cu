@@ -46,6 +46,7 @@
 #include <mutex>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 
 namespace tpb {
 namespace kernels {
@@ -422,7 +423,7 @@ __device__ __noinline__ void rowCopyTiles(const PushEntry& e, uint32_t first, ui
   const int64_t pitch = e.rowStride * e.srcElemSize;
   const uint64_t total = static_cast<uint64_t>(e.rows) * rowBytes;
   [[maybe_unused]] const uint64_t span = static_cast<uint64_t>(e.rows - 1) * pitch + rowBytes;
-  const uint32_t numTiles = e.numTiles, skew = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(dst) & 15);
+  const uint32_t numTiles = e.numTiles, tileBytes = e.rowTileBytes, skew = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(dst) & 15);
   const uint32_t stepRows = 512 / rowBytes, stepBytes = 512 - stepRows * rowBytes;  // 32 lanes x 16 bytes further on
   const int64_t stepPitch = pitch * stepRows;
   auto cursorAt = [&](uint64_t x) {
@@ -439,8 +440,8 @@ __device__ __noinline__ void rowCopyTiles(const PushEntry& e, uint32_t first, ui
   };
 #pragma unroll 1
   for (uint32_t t = first; t < numTiles; t += step) {
-    const uint64_t off = t == 0 ? 0 : static_cast<uint64_t>(t) * kPlainTileBytes - skew;
-    const uint64_t end = t + 1 == numTiles ? total : (static_cast<uint64_t>(t) + 1) * kPlainTileBytes - skew;
+    const uint64_t off = t == 0 ? 0 : static_cast<uint64_t>(t) * tileBytes - skew;
+    const uint64_t end = t + 1 == numTiles ? total : (static_cast<uint64_t>(t) + 1) * tileBytes - skew;
     const uint32_t bytes = static_cast<uint32_t>(end - off);
     uint32_t head = t == 0 ? (16 - skew) & 15 : 0;
     if (head > bytes) head = bytes;
@@ -475,30 +476,28 @@ __device__ __noinline__ void rowCopyTiles(const PushEntry& e, uint32_t first, ui
       if constexpr (kAligned) return *reinterpret_cast<const uint4*>(from.row + from.at);
       else return loadBytes16(from.row + from.at, 0, n);
     };
-    constexpr int U = kAligned ? 8 : 4;
+    auto batches = [&](auto size) {  // as many whole batches of vectors i, i + 32, ... as there are
+      constexpr int U = decltype(size)::value;
 #pragma unroll 1
-    for (; i + (U - 1) * 32 < vectors; i += U * 32) {
-      uint4 v[U];
-      RowCursor from[U];
+      for (; i + (U - 1) * 32 < vectors; i += U * 32) {
+        uint4 v[U];
+        RowCursor from[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        from[u] = c;
-        v[u] = load(c);
-        advance(c);
-      }
+        for (int u = 0; u < U; ++u) {
+          from[u] = c;
+          v[u] = load(c);
+          advance(c);
+        }
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if constexpr (!kAligned) v[u] = finish(v[u], from[u]);
-        if (TPB_DBG_INSIDE(out + i + u * 32, 16, dst, total)) out[i + u * 32] = v[u];
+        for (int u = 0; u < U; ++u) {
+          if constexpr (!kAligned) v[u] = finish(v[u], from[u]);
+          if (TPB_DBG_INSIDE(out + i + u * 32, 16, dst, total)) out[i + u * 32] = v[u];
+        }
       }
-    }
-#pragma unroll 1
-    for (; i < vectors; i += 32) {
-      uint4 v = load(c);
-      if constexpr (!kAligned) v = finish(v, c);
-      if (TPB_DBG_INSIDE(out + i, 16, dst, total)) out[i] = v;
-      advance(c);
-    }
+    };
+    batches(std::integral_constant<int, kAligned ? 8 : 4>());
+    batches(std::integral_constant<int, 2>());
+    batches(std::integral_constant<int, 1>());
   }
 }
 
@@ -508,8 +507,7 @@ template <typename S, typename D, int kUnit>
 __device__ __forceinline__ void rowCastTiles(const PushEntry& e, uint32_t first, uint32_t step, int lane) {
   struct alignas(kUnit * sizeof(S)) In { S v[kUnit]; };
   struct alignas(kUnit * sizeof(D)) Out { D v[kUnit]; };
-  constexpr uint32_t perTile = kPlainTileBytes / sizeof(D);
-  constexpr int U = 8;
+  const uint32_t perTile = e.rowTileBytes / static_cast<uint32_t>(sizeof(D));
   const S* const src = static_cast<const S*>(e.src);
   D* const dst = static_cast<D*>(e.dst);
   const uint32_t cols = static_cast<uint32_t>(e.cols), numTiles = e.numTiles;
@@ -545,16 +543,20 @@ __device__ __forceinline__ void rowCastTiles(const PushEntry& e, uint32_t first,
       if (TPB_DBG_INSIDE(out + i, sizeof(Out), dst, count * sizeof(D))) out[i] = o;
     };
     uint32_t i = lane;
+    auto batches = [&](auto size) {
+      constexpr int U = decltype(size)::value;
 #pragma unroll 1
-    for (; i + (U - 1) * 32 < units; i += U * 32) {
-      In v[U];
+      for (; i + (U - 1) * 32 < units; i += U * 32) {
+        In v[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) v[u] = load();
+        for (int u = 0; u < U; ++u) v[u] = load();
 #pragma unroll
-      for (int u = 0; u < U; ++u) storeConverted(v[u], i + u * 32);
-    }
-#pragma unroll 1
-    for (; i < units; i += 32) storeConverted(load(), i);
+        for (int u = 0; u < U; ++u) storeConverted(v[u], i + u * 32);
+      }
+    };
+    batches(std::integral_constant<int, 8>());
+    batches(std::integral_constant<int, 2>());
+    batches(std::integral_constant<int, 1>());
   }
 }
 template <typename S, typename D>
@@ -1882,7 +1884,7 @@ void pushEntry(PushPlan& plan, PushEntry e) {
     e.tileStart = plan.plainTiles;
     plan.plainTiles += e.numTiles;
   } else if (e.kind == kRows) {
-    e.numTiles = static_cast<uint32_t>((e.count * e.dstElemSize + kPlainTileBytes - 1) / kPlainTileBytes);
+    e.numTiles = static_cast<uint32_t>((e.count * e.dstElemSize + e.rowTileBytes - 1) / e.rowTileBytes);
     e.tileStart = plan.plainTiles;
     plan.plainTiles += e.numTiles;
   } else if (e.kind == kStridedBand) {
@@ -2006,7 +2008,10 @@ void appendToPlan(PushPlan& plan, const CopyItem& item, bool useBulk) {
       // would straddle more than two rows per vector: those, and rows whose length does not fit the
       // kernel's 32-bit offsets, stay with the element-wise tiles.
       const uint64_t srcRowBytes = static_cast<uint64_t>(v.cols) * e.srcElemSize;
-      if (v.rows > 1 && v.colStride == 1 && srcRowBytes >= 16 && srcRowBytes < (1u << 31) && (!convert || v.cols >= 16)) e.kind = kRows;
+      if (v.rows > 1 && v.colStride == 1 && srcRowBytes >= 16 && srcRowBytes < (1u << 31) && (!convert || v.cols >= 16)) {
+        e.kind = kRows;
+        e.rowTileBytes = rowTileBytes(static_cast<uint64_t>(v.rows) * dstRowBytes);
+      }
     }
     e.rows = v.rows;
     e.cols = v.cols;

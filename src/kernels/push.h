@@ -58,12 +58,21 @@ struct alignas(16) PushEntry {
   int64_t rows, cols, rowStride, colStride;  // kStrided only, in elements
   uint32_t tileStart;    // first tile of this entry within its class (bulk / plain)
   uint32_t numTiles;
+  uint32_t rowTileBytes; // kRows: bytes of the packed result in one tile
 };
 static_assert(sizeof(PushEntry) == 80, "entry layout");
 
 constexpr int kMaxEntriesSmall = 8;
 constexpr int kMaxEntriesLarge = 96;
 constexpr uint32_t kPlainTileBytes = 8 * 1024;  // one warp's unit of work (destination bytes)
+// kRows: bytes of the packed result in one tile: as many as leave a tile to every warp of 148 SMs, in sizes that are
+// whole batches of the 16 bytes x 32 lanes a warp loads at once (1, 2, 8 and 16 of them).
+// (Single launches, 32x32 tiles / 8 KiB row tiles / these: 1 MiB of 40-byte rows of int64 12.7 / 23.0 / 8.7 us, 1 MiB of 20-byte
+// rows of fp32 15.0 / 25.1 / 10.5, 64 KiB of them 10.7 / 16.8 / 8.6.)
+constexpr inline uint32_t rowTileBytes(uint64_t packedBytes) {
+  const uint64_t perWarp = (packedBytes + 148 * 16 - 1) / (148 * 16);
+  return perWarp <= 512 ? 512u : perWarp <= 1024 ? 1024u : perWarp <= 4096 ? 4096u : kPlainTileBytes;
+}
 constexpr int kStridedTile = 32;                // a warp transposes 32x32 elements (16x32 for 8-byte ones)
 constexpr int kWideTile = 64;                   // kStridedWide16: 64x64 two-byte elements per warp tile
 constexpr int kNarrowMaxCols = 64;              // kStridedNarrow: 32 rows x (<= 64) columns per warp tile

@@ -259,6 +259,29 @@ TPB_GPU_TEST(Kernel, ViewsWithContiguousRows, 1) {
   checkMessage({narrow, wide});
 }
 
+// The same at every size of tile that a result of such rows is cut into, and at the edges between them.
+TPB_GPU_TEST(Kernel, ViewsWithContiguousRowsAtEveryTileSize, 1) {
+  const int64_t warps = 148 * 16;
+  for (int64_t tile : {512, 1024, 2048, 4608, 7680, 8192})
+    for (int64_t cols : {4, 5, 16, 33}) {
+      const int64_t rows = warps * tile / (cols * 4);  // the last row at which this tile is taken, or next to it
+      std::vector<Spec> specs;
+      for (int64_t more : {-1, 0, 1}) {
+        Spec s;
+        s.from = s.to = DType::kF32;
+        s.rows = rows + more;
+        s.cols = cols;
+        s.strided = true;
+        s.rowStride = cols + (more < 0 ? 4 : 1);
+        s.srcOff = more < 0 ? 0 : 4;
+        s.dstOff = more > 0 ? 4 : 0;
+        specs.push_back(s);
+      }
+      if (cols >= 16) specs[0].to = specs[2].to = DType::kBF16, specs[2].dstOff = 2;
+      checkMessage(specs);
+    }
+}
+
 // Large transposed matrices, which a CTA transposes tile by tile: extents around the tiles (128 columns; 128,
 // 64 or 32 rows), narrow matrices whose tiles hold several chunks of rows, odd column strides and addresses,
 // every element size, every conversion; alone and beside a tensor on the bulk path.

@@ -234,3 +234,36 @@ TPB_TEST(Plan, MappingsAreKeyedByHandleAndAccessingDeviceAndIdleOnesAreClosed) {
   EXPECT_TRUE(cache.open(b, 0, nullptr, &why) == pinned);
   EXPECT_EQ(cache.closedCount(), uint64_t(closed.size()));
 }
+
+namespace {
+CopyItem matrix(uintptr_t src, DType t, int64_t rows, int64_t cols, int64_t rowStride, int64_t colStride) {
+  CopyItem c;
+  c.src = at(src);
+  c.dst = at(0x400000000);
+  c.srcDtype = c.dstDtype = t;
+  c.srcBytes = static_cast<uint64_t>(rows) * cols * dtypeSize(t);
+  c.strided = true;
+  c.view = StridedView{t, rows, cols, rowStride, colStride};
+  return c;
+}
+}  // namespace
+
+// The tiles of a view with contiguous rows: small ones for small results, so that they are spread over the chip, always
+// whole rounds of 16 bytes per lane, and as many as cover the result.
+TPB_TEST(Plan, RowTilesGrowWithTheResult) {
+  uint32_t before = 0;
+  for (int64_t rows = 2; rows < 3000000; rows = rows * 3 / 2 + 1) {
+    PushPlan plan;
+    appendToPlan(plan, matrix(0x100000000, DType::kF32, rows, 5, 9, 1), true);
+    const PushEntry& e = plan.entries.back();
+    EXPECT_EQ(int(e.kind), int(kRows));
+    EXPECT_TRUE(e.rowTileBytes % 512 == 0 && e.rowTileBytes >= 512 && e.rowTileBytes <= kPlainTileBytes);
+    EXPECT_TRUE(e.rowTileBytes >= before);
+    before = e.rowTileBytes;
+    const uint64_t total = static_cast<uint64_t>(rows) * 20;
+    EXPECT_TRUE(uint64_t(e.numTiles) * e.rowTileBytes >= total && uint64_t(e.numTiles - 1) * e.rowTileBytes < total);
+    EXPECT_EQ(plan.plainTiles, e.numTiles);
+    if (total >= (20u << 20)) EXPECT_EQ(e.rowTileBytes, kPlainTileBytes);
+    else EXPECT_TRUE(e.numTiles <= 148 * 16);
+  }
+}
