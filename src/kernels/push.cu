@@ -63,6 +63,9 @@ PushTuning initialTuning() {
   if (const char* e = std::getenv("TPB_PUSH_NARROW")) {
     if (e[0] >= '0' && e[0] <= '2' && e[1] == 0) t.narrowRows = static_cast<uint32_t>(e[0] - '0');
   }
+  if (const char* e = std::getenv("TPB_PUSH_BLOCK")) {
+    if (e[0] >= '0' && e[0] <= '2' && e[1] == 0) t.blockForm = static_cast<uint32_t>(e[0] - '0');
+  }
   // The shape of the bulk pipeline can be tried out without rebuilding; values that setPushTuning
   // would refuse are ignored.
   auto number = [](const char* name, uint32_t fallback) {
@@ -255,8 +258,8 @@ __device__ __forceinline__ __half fromFloat<__half>(float v) { return __float2ha
 // Bound by memory. The two ends of a tile may lie at any alignment relative to each other (a slice of
 // a flat buffer sent into a fresh allocation): warpCopyRun moves it with 16-byte loads and stores all
 // the same. Tiles meet on 16-byte boundaries of the destination, so only an entry's own ends are
-// ragged. (Five bf16
-// slices at odd offsets, 238 MB: 142 us with loads as wide as both ends' common alignment, 78 us now.)
+// ragged. (Five bf16 slices at odd offsets, 238 MB: 142 us with loads as wide as both ends' common
+// alignment, 78 us now.)
 template <bool kShifted>
 __device__ __forceinline__ void copyPlainTilesTyped(const PushEntry& e, uint32_t first, uint32_t step, int lane) {
   const uint8_t* from = static_cast<const uint8_t*>(e.src);
@@ -1868,56 +1871,101 @@ uint64_t convertedBytes(uint64_t srcBytes, DType s, DType d) {
 }
 
 namespace {
+uint32_t tilesOf(const PushEntry& e, uint32_t bulkTileBytes) {
+  auto over = [](uint64_t n, uint64_t tile) { return (n + tile - 1) / tile; };
+  uint64_t tiles = 0;
+  switch (e.kind) {
+    case kCopyBulk: tiles = over(e.count, bulkTileBytes); break;
+    case kCopyPlain: tiles = over(e.count, kPlainTileBytes); break;
+    case kCastPlain: tiles = over(e.count, kPlainTileBytes / e.dstElemSize); break;
+    case kRows: tiles = over(e.count * e.dstElemSize, e.rowTileBytes); break;
+    case kStridedBand: tiles = over(e.rows, bandRows(static_cast<uint64_t>(e.cols), e.dstElemSize)); break;
+    case kStridedNarrow: tiles = over(e.rows, kStridedTile); break;
+    case kTransposed: {
+      const bool narrow = e.cols <= kBlockNarrowCols;
+      const uint64_t rows = 256 / e.srcElemSize * (narrow ? kBlockSlots / e.cols : 1);
+      tiles = over(e.rows, rows) * (narrow ? 1 : over(e.cols, kBlockSlots));
+      break;
+    }
+    case kStridedWide16: tiles = over(e.rows, kWideTile) * over(e.cols, kWideTile); break;
+    default: tiles = over(e.rows, e.srcElemSize == 8 ? kStridedTile / 2 : kStridedTile) * over(e.cols, kStridedTile); break;
+  }
+  return static_cast<uint32_t>(tiles);
+}
 void pushEntry(PushPlan& plan, PushEntry e) {
   if (e.count == 0) return;
-  if (e.kind == kCopyBulk) {
-    e.numTiles = static_cast<uint32_t>((e.count + plan.bulkTileBytes - 1) / plan.bulkTileBytes);
-    e.tileStart = plan.bulkTiles;
-    plan.bulkTiles += e.numTiles;
-  } else if (e.kind == kCopyPlain) {
-    e.numTiles = static_cast<uint32_t>((e.count + kPlainTileBytes - 1) / kPlainTileBytes);
-    e.tileStart = plan.plainTiles;
-    plan.plainTiles += e.numTiles;
-  } else if (e.kind == kCastPlain) {
-    const uint64_t perTile = kPlainTileBytes / e.dstElemSize;
-    e.numTiles = static_cast<uint32_t>((e.count + perTile - 1) / perTile);
-    e.tileStart = plan.plainTiles;
-    plan.plainTiles += e.numTiles;
-  } else if (e.kind == kRows) {
-    e.numTiles = static_cast<uint32_t>((e.count * e.dstElemSize + e.rowTileBytes - 1) / e.rowTileBytes);
-    e.tileStart = plan.plainTiles;
-    plan.plainTiles += e.numTiles;
-  } else if (e.kind == kStridedBand) {
-    const uint32_t perBand = bandRows(static_cast<uint64_t>(e.cols), e.dstElemSize);
-    e.numTiles = static_cast<uint32_t>((e.rows + perBand - 1) / perBand);
-    e.tileStart = plan.plainTiles;
-    plan.plainTiles += e.numTiles;
-  } else if (e.kind == kStridedNarrow) {
-    e.numTiles = static_cast<uint32_t>((e.rows + kStridedTile - 1) / kStridedTile);
-    e.tileStart = plan.plainTiles;
-    plan.plainTiles += e.numTiles;
-  } else if (e.kind == kTransposed) {
-    const bool narrow = e.cols <= kBlockNarrowCols;
-    const uint64_t rows = 256 / e.srcElemSize * (narrow ? kBlockSlots / e.cols : 1);
-    const uint64_t tr = (e.rows + rows - 1) / rows, tc = narrow ? 1 : (e.cols + kBlockSlots - 1) / kBlockSlots;
-    e.numTiles = static_cast<uint32_t>(tr * tc);
-    e.tileStart = plan.blockTiles;
-    plan.blockTiles += e.numTiles;
-  } else if (e.kind == kStridedWide16) {
-    const uint64_t tr = (e.rows + kWideTile - 1) / kWideTile, tc = (e.cols + kWideTile - 1) / kWideTile;
-    e.numTiles = static_cast<uint32_t>(tr * tc);
-    e.tileStart = plan.plainTiles;
-    plan.plainTiles += e.numTiles;
-  } else {
-    const int tileRows = e.srcElemSize == 8 ? kStridedTile / 2 : kStridedTile;
-    const uint64_t tr = (e.rows + tileRows - 1) / tileRows, tc = (e.cols + kStridedTile - 1) / kStridedTile;
-    e.numTiles = static_cast<uint32_t>(tr * tc);
-    e.tileStart = plan.plainTiles;
-    plan.plainTiles += e.numTiles;
-  }
+  uint32_t* const totals[kTileClasses] = {&plan.plainTiles, &plan.bulkTiles, &plan.blockTiles};
+  uint32_t& total = *totals[tileClassOf(e.kind)];
+  e.numTiles = tilesOf(e, plan.bulkTileBytes);
+  e.tileStart = total;
+  total += e.numTiles;
   plan.entries.push_back(e);
 }
+
 }  // namespace
+
+// Why the lines lie where they do. (Launches back to back on one B200, us each, warp form / block form; they end on steps
+// of about 2 us, so less than that is a tie.)
+//   * Few columns leave most lanes of a 32x32 warp tile idle, and a tile that is not quite full takes the warps' predicated
+//     path: 64 MiB of fp32 in 5 columns 178 / 32, 31 columns 77 / 33, 63 columns 78 / 31, 127 columns 72 / 28.
+//   * Where all warp tiles are full the block form only wins by its longer pieces, once there are tiles enough: fp32 in 128
+//     columns 8 MiB 8.3 / 10.3, 16 MiB 12.3 / 12.3, 64 MiB 35 / 27; in 64 columns 16 MiB 12.3 / 13.4, 64 MiB 34 / 31.
+//   * A last tile of few columns costs nearly a full one, most of all where the warp form writes less than it reads:
+//     64 MiB of fp32 -> bf16 in 65 columns 40 / 51, 129 columns 36 / 45, 160 columns 33 / 39, 257 columns 33 / 35.
+//   * Beside the bulk pipeline it has one stage and eight warps of one CTA an SM, and loses what it wins by overlap:
+//     64 MiB of fp32 beside 1 MiB, 64 columns 37 / 53, 130 columns 41 / 82, 1000 columns 39 / 53, but 5 columns 189 / 55,
+//     63 columns 82 / 56, 127 columns 82 / 51, 383 columns 77 / 51. The more the bulk pipeline has to do, the less it
+//     matters, and wide 2-byte matrices then gain: 16 MiB in 130 columns beside 16 MiB 29 / 31, beside 64 MiB 42 / 39.
+bool blockFormPays(const PushEntry& e, uint64_t bulkBytes) {
+  constexpr uint64_t MiB = 1 << 20, kNever = ~0ull;
+  const uint64_t bytes = e.count * e.srcElemSize;
+  const int64_t cols = e.cols;
+  const bool narrow = cols < kBlockNarrowCols, converts = e.srcElemSize != e.dstElemSize, widens = e.dstElemSize > e.srcElemSize;
+  // The share of a block tile's slots that hold a column; how many columns lie in a warp tile that is not full.
+  const double filled = cols <= kBlockNarrowCols ? static_cast<double>(kBlockSlots / cols * cols) / kBlockSlots
+                                                 : static_cast<double>(cols) / ((cols + kBlockSlots - 1) / kBlockSlots * kBlockSlots);
+  const int64_t ragged = cols % kStridedTile;
+  if (!widens && static_cast<uint64_t>(e.rows) * e.srcElemSize <= kBlockMinRowBytes) return false;
+
+  if (bulkBytes > 0) {
+    if ((cols > kBlockSlots || (cols > kBlockNarrowCols && filled >= 0.75)) && e.srcElemSize == 2 && !converts && bulkBytes >= 2 * bytes) return true;
+    if (ragged == 0) return false;
+    if (narrow) return e.srcElemSize == 2 || ragged > 2 || bytes >= 12 * MiB;
+    if (ragged > 24) return widens || !converts || filled >= 0.9;
+    return (filled >= 0.9 && bytes < 6 * MiB) || (widens && filled >= 0.75);
+  }
+
+  uint64_t least = 0;  // the plan has its own least size
+  if (cols == kStridedTile || cols == kBlockNarrowCols) {  // one or two warp tiles, all full
+    if (e.srcElemSize != 2) least = (e.srcElemSize == 8 ? 12 : converts ? 48 : 24) * MiB;
+    else least = widens ? 6 * MiB : cols == kBlockNarrowCols ? 48 * MiB : 0;
+  } else if (!narrow && e.srcElemSize != 2 && ragged < kStridedTile / 2) {
+    const bool full = ragged == 0 && (e.rows % kStridedTile == 0 || e.rows >= 10 * kStridedTile), several = cols > kBlockSlots;
+    if (converts && filled < (full ? 0.8 : several ? 0.7 : 0.6)) least = kNever;
+    else if (full) least = (filled < 0.66 ? 48 : 12) * MiB;
+    else if (several && filled < 0.6) least = e.srcElemSize == 8 ? 24 * MiB : kNever;
+    else if (several && filled < 0.7) least = 6 * MiB;
+  }
+  return bytes >= least;
+}
+
+std::vector<PushEntry> entriesOfLaunch(const PushEntry* entries, size_t n, uint32_t bulkTileBytes, uint32_t (&tiles)[kTileClasses]) {
+  std::vector<PushEntry> part(entries, entries + n);
+  const uint32_t blockForm = getPushTuning().blockForm;
+  uint64_t bulkBytes = 0;
+  for (const auto& e : part)
+    if (e.kind == kCopyBulk) bulkBytes += e.count;
+  for (auto& e : part) {
+    if (e.kind == kTransposed && (blockForm == 0 || (blockForm == 1 && !blockFormPays(e, bulkBytes)))) {
+      e.kind = e.warpForm;
+      e.numTiles = tilesOf(e, bulkTileBytes);
+    }
+    uint32_t& next = tiles[tileClassOf(e.kind)];
+    e.tileStart = next;
+    next += e.numTiles;
+  }
+  return part;
+}
 
 namespace {
 // Memory that the driver places on another GPU than the current one, or on the host.
@@ -2003,7 +2051,7 @@ void appendToPlan(PushPlan& plan, const CopyItem& item, bool useBulk) {
       if (useBulk && e.kind != kStridedNarrow && e.kind != kStridedBand && e.srcElemSize >= 2 && v.rowStride == 1 &&
           v.colStride != 1 && v.cols >= 2 && static_cast<uint64_t>(v.rows) * e.srcElemSize >= kBlockMinRowBytes &&
           item.srcBytes >= blockMinBytes(v.cols, e.srcElemSize) && smemWithWide <= kMaxSmemPerCta && !sourceIsForeign(item.src))
-        e.kind = kTransposed;
+        e.warpForm = e.kind, e.kind = kTransposed;
       // Rows that are contiguous in the source are copied as the runs they are. Shorter than a vector they
       // would straddle more than two rows per vector: those, and rows whose length does not fit the
       // kernel's 32-bit offsets, stay with the element-wise tiles.
@@ -2087,12 +2135,20 @@ int launchPush(const PushPlan& plan, cudaStream_t stream, int maxCtas, uint32_t*
   const uint32_t tileBytes = plan.bulkTileBytes ? plan.bulkTileBytes : 32768;
   const uint32_t stages = plan.bulkStages ? plan.bulkStages : 4;
   if (n <= static_cast<size_t>(kMaxEntriesLarge)) {
+    const PushEntry* entries = plan.entries.data();
+    uint32_t tiles[kTileClasses] = {plan.plainTiles, plan.bulkTiles, plan.blockTiles};
+    std::vector<PushEntry> part;
+    if (plan.blockTiles > 0) {
+      for (uint32_t& t : tiles) t = 0;
+      part = entriesOfLaunch(entries, n, tileBytes, tiles);
+      entries = part.data();
+    }
     if (n <= static_cast<size_t>(kMaxEntriesSmall))
-      launchOne<kMaxEntriesSmall>(plan.entries.data(), static_cast<uint32_t>(n), plan.bulkTiles, plan.plainTiles, plan.blockTiles,
+      launchOne<kMaxEntriesSmall>(entries, static_cast<uint32_t>(n), tiles[kBulkClass], tiles[kPlainClass], tiles[kBlockClass],
                                   tileBytes, stages, stream, maxCtas, flag, flagValue, counter, status, wait, done,
                                   plan.totalBytesOut);
     else
-      launchOne<kMaxEntriesLarge>(plan.entries.data(), static_cast<uint32_t>(n), plan.bulkTiles, plan.plainTiles, plan.blockTiles,
+      launchOne<kMaxEntriesLarge>(entries, static_cast<uint32_t>(n), tiles[kBulkClass], tiles[kPlainClass], tiles[kBlockClass],
                                   tileBytes, stages, stream, maxCtas, flag, flagValue, counter, status, wait, done,
                                   plan.totalBytesOut);
     return 1;
@@ -2102,13 +2158,8 @@ int launchPush(const PushPlan& plan, cudaStream_t stream, int maxCtas, uint32_t*
   int launches = 0;
   for (size_t first = 0; first < n; first += kMaxEntriesLarge) {
     const size_t cnt = n - first < static_cast<size_t>(kMaxEntriesLarge) ? n - first : kMaxEntriesLarge;
-    std::vector<PushEntry> part(plan.entries.begin() + first, plan.entries.begin() + first + cnt);
     uint32_t tiles[kTileClasses] = {};
-    for (auto& e : part) {
-      uint32_t& next = tiles[tileClassOf(e.kind)];
-      e.tileStart = next;
-      next += e.numTiles;
-    }
+    const std::vector<PushEntry> part = entriesOfLaunch(plan.entries.data() + first, cnt, tileBytes, tiles);
     const bool last = first + cnt == n;
     // Only the first launch waits for the producer; stream order covers the rest.
     launchOne<kMaxEntriesLarge>(part.data(), static_cast<uint32_t>(cnt), tiles[kBulkClass], tiles[kPlainClass],

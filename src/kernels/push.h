@@ -52,13 +52,14 @@ constexpr inline bool isView(uint32_t kind) { return kind != kCopyBulk && kind !
 struct alignas(16) PushEntry {
   const void* src;
   void* dst;
-  uint64_t count;        // bytes for kCopy*, elements for kCast*/kStrided (= rows*cols)
+  uint64_t count;        // bytes for kCopy*, elements for kCast* and all views (= rows*cols)
   uint32_t kind;
   uint8_t srcDtype, dstDtype, srcElemSize, dstElemSize;
-  int64_t rows, cols, rowStride, colStride;  // kStrided only, in elements
-  uint32_t tileStart;    // first tile of this entry within its class (bulk / plain)
+  int64_t rows, cols, rowStride, colStride;  // views only, in elements
+  uint32_t tileStart;    // first tile of this entry within its class (bulk / plain / block)
   uint32_t numTiles;
   uint32_t rowTileBytes; // kRows: bytes of the packed result in one tile
+  uint32_t warpForm;     // kTransposed: the form (EntryKind) whose tiles one warp takes alone
 };
 static_assert(sizeof(PushEntry) == 80, "entry layout");
 
@@ -87,14 +88,17 @@ constexpr inline uint32_t bandRows(uint64_t cols, uint32_t dstElemSize) {
 constexpr int kBlockSlots = 128;
 constexpr int kBlockNarrowCols = 64;
 constexpr uint64_t kBlockMinRowBytes = 128;  // shorter columns would leave most of a slot empty
-// From which size on it pays: below, there are too few tiles of 32 KiB for the SMs and the warp tiles finish first
+                                             // (32 MiB of fp32, warp tiles / this: columns of 128 bytes, one full warp
+                                             // tile high, 18.6 / 22.6 us; of 136 bytes 33.7 / 22.6, of 160 30.6 / 21.3)
+// From which size on it can pay: below, there are too few tiles of 32 KiB for the SMs and the warp tiles finish first
 // (kernel times, warp tiles / this: fp32 of 2 MiB 8.6-11 / 9 us and 16 MiB 13.2 / 11.6; 8 columns of 4 MiB 14 / 9;
 // wide 2-byte matrices, where a tile takes the longest to write, 4 MiB 10.8 / 14.1, 8 MiB 12.5 / 12.6, 16 MiB 22 / 18).
+// Above, blockFormPays decides.
 constexpr inline uint64_t blockMinBytes(uint64_t cols, uint32_t srcElemSize) {
   return srcElemSize == 2 && cols > kBlockNarrowCols ? 8u << 20 : 4u << 20;
 }
 constexpr int kThreads = 512;                   // full kernel: warp 0 drives TMA, warps 1..15 use registers
-constexpr int kLightThreads = 256;              // light kernel (no bulk pipeline, static shared memory only)
+constexpr int kLightThreads = 256;              // light kernel (no bulk copy engine; dynamic shared memory for staged views only)
 constexpr int kMaxBulkStages = 8;
 
 // Shape of the TMA bulk pipeline; process-wide, read when a plan is built. The defaults are the
@@ -110,6 +114,9 @@ struct PushTuning {
   // (kStridedBand), wherever the narrow form above does not apply: 0 never, 1 for remote
   // destinations (default), 2 always. TPB_PUSH_BAND overrides the default.
   uint32_t bandRows = 1;
+  // Large transposed matrices moved as CTA tiles (kTransposed): 0 never, 1 where that is the faster form (default), 2
+  // wherever it is possible. TPB_PUSH_BLOCK overrides the default.
+  uint32_t blockForm = 1;
 };
 void setPushTuning(const PushTuning& t);
 PushTuning getPushTuning();
@@ -158,6 +165,16 @@ void chooseBulkTile(PushPlan& plan, uint64_t bulkBytes, int ctas);
 // Splits items into kernel entries (aligned body for the bulk path, ragged head/tail for the
 // plain path) and numbers their tiles. `useBulk=false` routes everything through the plain path.
 void appendToPlan(PushPlan& plan, const CopyItem& item, bool useBulk);
+
+// Whether the block form of a kTransposed entry is faster than its warp form, alone (bulkBytes 0) or in a launch whose
+// bulk pipeline moves that many bytes.
+bool blockFormPays(const PushEntry& e, uint64_t bulkBytes);
+
+// Entries that go into one launch, as that launch runs them: the tiles of each class numbered from 0 (`tiles`,
+// zeroed by the caller, counts them), and kTransposed entries whose block form does not pay in their warp form. (For
+// the launcher and for tests.)
+std::vector<PushEntry> entriesOfLaunch(const PushEntry* entries, size_t n, uint32_t bulkTileBytes,
+                                       uint32_t (&tiles)[kTileClasses]);
 
 // A launch may be told to hold back until a flag that another GPU writes has reached a value
 // (cyclic comparison, as tpb_wait_flag does), for at most timeoutNs; on a timeout it copies

@@ -76,7 +76,7 @@ struct DeviceMem {
 };
 
 // All specs as one message: one plan, checked element by element; gaps must keep their canaries.
-void checkMessage(const std::vector<Spec>& specs, bool bulk = true, int ctas = 148) {
+void checkMessage(const std::vector<Spec>& specs, bool bulk = true, int ctas = 148, bool publish = false) {
   std::mt19937 rng(static_cast<uint32_t>(specs.size() * 977 + specs[0].cols * 31 + specs[0].srcOff));
   size_t srcBytes = 256, dstBytes = 256;
   std::vector<size_t> srcAt, dstAt;
@@ -121,7 +121,19 @@ void checkMessage(const std::vector<Spec>& specs, bool bulk = true, int ctas = 1
         else store(to, s.to, valueOf(from, s.from));
       }
   }
-  if (!plan.entries.empty()) launchPush(plan, nullptr, ctas, nullptr, 0, nullptr, nullptr);
+  if (publish) {
+    DeviceMem words(256);  // flag, arrive counter, status
+    CK(cudaMemset(words.p, 0, 256));
+    uint32_t* w = reinterpret_cast<uint32_t*>(words.p);
+    launchPush(plan, nullptr, ctas, w, 77, w + 8, w + 16);
+    uint32_t after[64];
+    CK(cudaMemcpy(after, words.p, 256, cudaMemcpyDeviceToHost));
+    EXPECT_EQ(after[0], uint32_t(77));
+    EXPECT_EQ(after[8], uint32_t(0));
+    EXPECT_EQ(after[16], uint32_t(kStatusOk));
+  } else if (!plan.entries.empty()) {
+    launchPush(plan, nullptr, ctas, nullptr, 0, nullptr, nullptr);
+  }
   CK(cudaDeviceSynchronize());
   CK(cudaMemcpy(got.data(), ddst.p, got.size(), cudaMemcpyDeviceToHost));
   if (got != want) {
@@ -368,4 +380,43 @@ TPB_GPU_TEST(Kernel, LargeTransposedMatricesInOneMessage, 1) {
   specs.push_back(bulk);         // the full one: eight of its warps share the block tiles
   checkMessage(specs);
   checkMessage(specs, true, 3);
+}
+
+// More entries than one launch takes: both sides of the cut hold transposed matrices, contiguous rows and plain runs, and
+// the tiles of each launch are numbered anew. The flag is published once, behind all of them.
+TPB_GPU_TEST(Kernel, MessagesOfMoreThanOneLaunch, 1) {
+  for (bool withBulk : {false, true}) {
+    std::vector<Spec> specs;
+    for (int i = 0; i < 130; ++i) {
+      if (i == 3 || i == 95 || i == 96 || i == 120) {
+        specs.push_back(transposed(DType::kF32, i == 96 ? DType::kBF16 : DType::kF32, i == 3 ? 180001 : 4099, i == 3 ? 7 : 259 + i, 1, 0, i & 1));
+      } else if (i % 10 == 5) {
+        Spec s;
+        s.from = s.to = DType::kI64;
+        s.rows = 100 + i;
+        s.cols = 5 + i % 3;
+        s.strided = true;
+        s.rowStride = s.cols + 2;
+        specs.push_back(s);
+      } else if (withBulk && (i == 50 || i == 110)) {
+        specs.push_back(run(1 << 20, 0, 0));
+      } else {
+        specs.push_back(run(1000 + 37 * i, i % 16, (i * 7) % 16));
+      }
+    }
+    checkMessage(specs, true, 148, true);
+    checkMessage(specs, true, 5, true);
+  }
+}
+
+// A column that stands for all (stride 0), as an expanded tensor has it.
+TPB_GPU_TEST(Kernel, TransposedMatricesOfOneRepeatedColumn, 1) {
+  for (int64_t cols : {3, 64, 129}) {
+    Spec s = transposed(DType::kF32, DType::kF32, (5 << 20) / 4 / cols, cols, 0, 1, 0);
+    s.colStride = 0;
+    EXPECT_EQ(int(kindOf(s)), int(kTransposed));
+    checkMessage({s});
+    s.to = DType::kBF16;
+    checkMessage({s, run(1 << 20, 0, 0)});
+  }
 }

@@ -248,6 +248,75 @@ CopyItem matrix(uintptr_t src, DType t, int64_t rows, int64_t cols, int64_t rowS
 }
 }  // namespace
 
+// A large transposed matrix is run in the block form or in its warp form, whichever is faster for its extents, its type
+// and what the bulk pipeline has to do; the order of the tensors does not matter, and nothing else about the entries
+// changes. The tuning can ask for either.
+TPB_TEST(Plan, TransposedMatricesTakeTheFasterForm) {
+  struct Case {
+    DType from, to;
+    int64_t rows, cols;
+    uint32_t warp;
+    bool alone, beside;  // block form
+  };
+  const DType F32 = DType::kF32, BF = DType::kBF16, I64 = DType::kI64;
+  const PushTuning tuned = getPushTuning();
+  for (const Case& c : {Case{F32, F32, 1 << 17, 9, kStrided, true, true}, Case{F32, F32, 1 << 16, 43, kStrided, true, true}, Case{F32, F32, 40000, 33, kStrided, true, false},
+                        Case{BF, BF, 1 << 17, 43, kStrided, true, true}, Case{F32, F32, 1 << 16, 32, kStrided, false, false}, Case{F32, F32, 1 << 18, 32, kStrided, true, false},
+                        Case{F32, F32, 1 << 16, 63, kStrided, true, true},
+                        Case{F32, F32, 65536, 64, kStrided, false, false}, Case{F32, F32, 100000, 64, kStrided, true, false},
+                        Case{F32, F32, 1100, 1000, kStrided, true, true}, Case{F32, F32, 4096, 1000, kStrided, true, false},
+                        Case{F32, F32, 4096, 512, kStrided, false, false}, Case{F32, F32, 8192, 512, kStrided, true, false},
+                        Case{I64, I64, 10000, 129, kStrided, false, false}, Case{I64, I64, 30000, 129, kStrided, true, false},
+                        Case{F32, BF, 200000, 65, kStrided, false, false}, Case{F32, BF, 200000, 127, kStrided, true, true}, Case{F32, F32, 32, 300000, kStrided, false, false},
+                        Case{BF, F32, 100000, 65, kStrided, true, false}, Case{BF, F32, 40000, 64, kStrided, false, false},
+                        Case{BF, BF, 8192, 1024, kStridedWide16, true, false}, Case{BF, BF, 8191, 1023, kStrided, true, true}, Case{BF, BF, 8191, 1025, kStrided, true, false},
+                        Case{BF, BF, 1 << 18, 64, kStridedWide16, false, false}, Case{F32, F32, 16384, 600, kStrided, true, false},
+                        Case{F32, F32, 100000, 159, kStrided, true, true}, Case{F32, BF, 100000, 159, kStrided, true, false},
+                        Case{BF, F32, 64, 100000, kStrided, true, false}})
+    for (uint32_t asked : {0u, 1u, 2u})
+      for (int withBulk = 0; withBulk < 3; ++withBulk) {  // without, in front, behind
+        PushTuning t = tuned;
+        t.blockForm = asked;
+        setPushTuning(t);
+        CopyItem m = matrix(0x100000000, c.from, c.rows, c.cols, 1, c.rows);
+        m.dstDtype = c.to;
+        PushPlan plan;
+        if (withBulk == 1) appendToPlan(plan, contiguous(0x10000000, 0x20000000, 1 << 20), true);
+        appendToPlan(plan, m, true);
+        appendToPlan(plan, contiguous(0x30000000, 0x30800001, 100000), true);
+        if (withBulk == 2) appendToPlan(plan, contiguous(0x10000000, 0x20000000, 1 << 20), true);
+        uint32_t tiles[kTileClasses] = {};
+        const std::vector<PushEntry> run = entriesOfLaunch(plan.entries.data(), plan.entries.size(), plan.bulkTileBytes, tiles);
+        setPushTuning(tuned);
+        EXPECT_EQ(run.size(), plan.entries.size());
+        const bool block = asked == 2 || (asked == 1 && (withBulk ? c.beside : c.alone));
+        uint32_t next[kTileClasses] = {};
+        for (size_t i = 0; i < run.size(); ++i) {
+          const PushEntry& e = run[i];
+          if (isView(e.kind)) {
+            if (int(e.kind) != int(block ? kTransposed : c.warp))
+              throw tpbtest::TestFailure(std::to_string(c.rows) + "x" + std::to_string(c.cols) + " type " + std::to_string(int(c.from)) + "->" +
+                                         std::to_string(int(c.to)) + (withBulk ? " beside bulk" : " alone") + ": form " + std::to_string(e.kind));
+          } else {
+            EXPECT_EQ(int(e.kind), int(plan.entries[i].kind));
+          }
+          EXPECT_TRUE(e.src == plan.entries[i].src && e.dst == plan.entries[i].dst && e.count == plan.entries[i].count);
+          EXPECT_EQ(e.tileStart, next[tileClassOf(e.kind)]);
+          next[tileClassOf(e.kind)] += e.numTiles;
+          if (e.kind == kStrided) {
+            const int64_t high = e.srcElemSize == 8 ? kStridedTile / 2 : kStridedTile;
+            EXPECT_EQ(int64_t(e.numTiles), ((c.rows + high - 1) / high) * ((c.cols + kStridedTile - 1) / kStridedTile));
+          }
+        }
+        for (int k = 0; k < kTileClasses; ++k) EXPECT_EQ(tiles[k], next[k]);
+      }
+  // A bulk pipeline with enough to do leaves the warps time: wide matrices of 2-byte elements keep the block form.
+  PushPlan plan;
+  appendToPlan(plan, matrix(0x100000000, BF, 65000, 132, 1, 65000), true);
+  EXPECT_TRUE(blockFormPays(plan.entries[0], 40u << 20));
+  EXPECT_TRUE(!blockFormPays(plan.entries[0], 20u << 20));
+}
+
 // The tiles of a view with contiguous rows: small ones for small results, so that they are spread over the chip, always
 // whole rounds of 16 bytes per lane, and as many as cover the result.
 TPB_TEST(Plan, RowTilesGrowWithTheResult) {
