@@ -3,10 +3,11 @@
 Some callers of this library cannot call cudaMalloc: a serving loop that must not trigger the
 device-wide synchronisation an allocation implies, a plugin living inside a fixed memory budget, a
 process whose framework already owns all device memory. For them the library exports
-`tpb_noalloc_push`, whose scratch memory is a fixed array inside the library image. This test calls
-it through its exported C symbol (ctypes, no Python binding in between) and checks that it moves
-exactly the bytes the ordinary entry point moves, twice in a row, because the second call finds the
-first call's table and counter still in the shared array.
+`tpb_noalloc_push`: its table of copies travels as the kernel's parameter (a short and a long form), and its arrive
+counters are a fixed array inside the library image, which calls take in turn and leave at zero. These tests call
+it through its exported C symbol (ctypes, no Python binding in between) and check that it moves
+exactly the bytes the ordinary entry point moves, at the edges of both forms, and that every one of many calls
+back to back publishes its flag.
 
 This file is collected last on purpose: should it fail, a run that stops at the first failure has
 already run every other test.
@@ -88,3 +89,66 @@ def test_no_alloc_entry_point_matches_the_ordinary_kernel(built):
     assert rc == 0
     torch.cuda.synchronize()
     assert int(flags[3]) == 99
+
+
+def table_of(count, g):
+    """`count` non-empty ranges of ragged lengths at odd offsets, with empty ones in between where the table has room."""
+    sizes = [1, 15, 16, 17, 700, 4099, 8192, 8193, 40001]
+    out, src_off, dst_off = [], 0, 0
+    spare = MAX_ITEMS - count
+    for i in range(count):
+        if spare and i % 5 == 2:
+            out.append((src_off, dst_off, 0))
+            spare -= 1
+        n = sizes[int(torch.randint(0, len(sizes), (1,), generator=g))] + i % 3
+        out.append((src_off + int(torch.randint(0, 16, (1,), generator=g)), dst_off + int(torch.randint(0, 16, (1,), generator=g)), n))
+        src_off += n + 32
+        dst_off += n + 48
+    return out, src_off, dst_off
+
+
+def push(fn, strerror, src, dst, triples, flag, value, stream):
+    arr = (Item * len(triples))(*[Item(src.data_ptr() + s, dst.data_ptr() + d, n) for s, d, n in triples])
+    rc = fn(arr, len(triples), flag.data_ptr(), value, stream)
+    assert rc == 0, strerror(rc).decode()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("count", [1, 2, 15, 16, 17, 128, 255, 256])
+def test_no_alloc_tables_of_every_size(built, count):
+    """Both forms of the kernel, at the edges of their tables: every byte of every range and not one besides."""
+    fn, strerror = load_symbol()
+    stream = torch.cuda.current_stream().cuda_stream
+    triples, src_total, dst_total = table_of(count, torch.Generator().manual_seed(count))
+    assert len(triples) <= MAX_ITEMS and sum(n > 0 for _, _, n in triples) == count
+    src = torch.randint(0, 256, (src_total,), dtype=torch.uint8, device="cuda")
+    got = torch.full((dst_total,), 0xCD, dtype=torch.uint8, device="cuda")
+    flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+    push(fn, strerror, src, got, triples, flag, count, stream)
+    torch.cuda.synchronize()
+    expect, from_ = torch.full((dst_total,), 0xCD, dtype=torch.uint8), src.cpu()
+    for s, d, n in triples:
+        expect[d:d + n] = from_[s:s + n]
+    assert torch.equal(got.cpu(), expect)
+    assert int(flag[0]) == count
+
+
+@pytest.mark.gpu
+def test_no_alloc_calls_back_to_back_publish_every_flag(built):
+    """More calls than there are arrive counters (64), of several thread blocks each, in both forms: a counter that a
+    call did not leave at zero would lose the flag of the call that is given it next."""
+    fn, strerror = load_symbol()
+    stream = torch.cuda.current_stream().cuda_stream
+    calls = 200
+    src = torch.randint(0, 256, (400_000,), dtype=torch.uint8, device="cuda")
+    got = torch.zeros(calls, 400_000, dtype=torch.uint8, device="cuda")
+    flags = torch.zeros(calls, dtype=torch.int32, device="cuda")
+    for i in range(calls):
+        parts = 3 if i % 3 else 20
+        n = 400_000 // parts
+        push(fn, strerror, src, got[i], [(k * n, k * n, n) for k in range(parts)], flags[i:], 1000 + i, stream)
+    torch.cuda.synchronize()
+    assert flags.tolist() == list(range(1000, 1000 + calls))
+    for i in range(calls):
+        whole = 400_000 // (3 if i % 3 else 20) * (3 if i % 3 else 20)
+        assert torch.equal(got[i, :whole], src[:whole]) and not bool(got[i, whole:].any())
