@@ -466,6 +466,8 @@ PYBIND11_MODULE(_C, m) {
       });
 
   m.def("kernel_launch_count", &kernels::launchCount);
+  m.def("tensor_record", [](const std::string& dtype, py::tuple shape) { return py::bytes(tensorRecord(dtype, shape)); },
+        "The metadata that the Python layer attaches to a tensor.");
   m.def("trace_enable", &traceEnable, py::arg("path"),
         "Start recording pipe / channel / kernel-launch events; trace_dump() writes chrome://tracing JSON.");
   m.def("trace_disable", &traceDisable);

@@ -43,8 +43,9 @@ def kernel_launch_count() -> int:
 
 def _parse_tensor_metadata(raw: bytes):
     """(dtype name, shape) out of the metadata this module attaches to tensors, or None for anything
-    else (a foreign peer's metadata). The exact bytes `_add_tensor` writes are recognised without a
-    JSON parser; anything that merely is JSON with those two keys still goes through json."""
+    else (a foreign peer's metadata). Called for what the native reader did not recognise as a record of this
+    library: records in much the same form without a JSON parser, anything else that is JSON with those two keys
+    through json."""
     if raw.startswith(b'{"dtype": "') and raw.endswith(b']}'):
         try:
             end = raw.index(b'"', 11)
@@ -185,9 +186,8 @@ class Pipe:
     def _add_raw(self, out, t: torch.Tensor, ptr: int, device: torch.device, target: Optional[str],
                  metadata: Optional[bytes], streams: Optional[Dict[torch.device, int]], view) -> None:
         """Adds `t` as a tensor that the library reads at `ptr` on behalf of `device`."""
-        meta = metadata if metadata is not None else (
-            '{"dtype": "%s", "shape": %s}' % (_DTYPE_NAMES.get(t.dtype) or str(t.dtype).replace("torch.", ""),
-                                              list(t.shape))).encode()
+        meta = metadata if metadata is not None else _C.tensor_record(
+            _DTYPE_NAMES.get(t.dtype) or str(t.dtype).replace("torch.", ""), tuple(t.shape))
         dev_type, dev_index = _device_str(device).split(":")
         if streams is None:
             stream = _stream_handle(device)
