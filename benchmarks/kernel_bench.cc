@@ -201,6 +201,66 @@ int main(int argc, char** argv) {
     report("cudaMemcpyAsync pinned host -> device", total, ms);
     cudaFreeHost(pinned);
   }
+  if (want("forms")) {
+    // The forms that a message of few large tensors meets: slices at odd offsets, conversions, columns of a matrix,
+    // transposed matrices. Read + written bytes per second; `bytes` must hold the largest (512 MiB).
+    struct Item {
+      DType from, to;
+      int64_t rows, cols, rowStride, colStride;  // elements; rows 1 for a contiguous run
+      size_t srcOff;
+    };
+    auto run = [](DType from, DType to, int64_t n, size_t off = 0) { return Item{from, to, 1, n, n, 1, off}; };
+    auto columns = [](DType from, DType to, int64_t rows, int64_t cols, int64_t pitch) { return Item{from, to, rows, cols, pitch, 1, 0}; };
+    auto transposed = [](DType from, DType to, int64_t rows, int64_t cols) { return Item{from, to, rows, cols, 1, rows, 0}; };
+    const DType F = DType::kF32, B = DType::kBF16, L = DType::kI64;
+    const int64_t M = 1 << 20, d = 4096;
+    std::vector<Item> odd, narrowing, widening;
+    for (int64_t n : {50 * M + 1, 3 * M, int64_t(1023), 40 * M + 5, 20 * M + 3}) odd.push_back(run(B, B, n, 2));
+    for (int64_t n : {3 * d * d, 3 * d, d * d, d, 4 * d * d, 4 * d, 4 * d * d, d, d, d, d, d}) {
+      narrowing.push_back(run(F, B, n));
+      widening.push_back(run(B, F, n));
+    }
+    const std::vector<std::pair<const char*, std::vector<Item>>> forms = {
+        {"five bf16 slices, 2 bytes off", odd},
+        {"transformer layer fp32 -> bf16", narrowing},
+        {"transformer layer bf16 -> fp32", widening},
+        {"4 x 16384 x 2048 of 8192 columns, bf16", std::vector<Item>(4, columns(B, B, 16384, 2048, 8192))},
+        {"4 x 16384 x 2047 of 8191 columns, bf16", std::vector<Item>(4, columns(B, B, 16384, 2047, 8191))},
+        {"4 x 16384 x 2048 of 8192, bf16 -> fp32", std::vector<Item>(4, columns(B, F, 16384, 2048, 8192))},
+        {"2 x 16384 x 2048 of 8192, fp32 -> bf16", std::vector<Item>(2, columns(F, B, 16384, 2048, 8192))},
+        {"2 x 8192 x 8192 fp32 transposed", std::vector<Item>(2, transposed(F, F, 8192, 8192))},
+        {"4 x 8191 x 4097 bf16 transposed", std::vector<Item>(4, transposed(B, B, 8191, 4097))},
+        {"2 x 8192 x 4096 int64 transposed", std::vector<Item>(2, transposed(L, L, 8192, 4096))},
+        {"8192 x 8192 fp32 -> bf16 transposed", std::vector<Item>(1, transposed(F, B, 8192, 8192))},
+        {"2 x 4 Mi x 8 fp32 transposed", std::vector<Item>(2, transposed(F, F, 4 * M, 8))},
+        {"2 x 1 Mi x 50 bf16 transposed", std::vector<Item>(2, transposed(B, B, M, 50))},
+    };
+    for (const auto& form : forms) {
+      PushPlan plan;
+      uint64_t srcOff = 0, dstOff = 0, moved = 0;
+      for (const Item& i : form.second) {
+        CopyItem it;
+        it.src = src + srcOff + i.srcOff;
+        it.dst = dst + dstOff;
+        it.srcDtype = i.from;
+        it.dstDtype = i.to;
+        it.srcBytes = static_cast<uint64_t>(i.rows) * i.cols * dtypeSize(i.from);
+        if (i.rows > 1) {
+          it.strided = true;
+          it.view = StridedView{i.from, i.rows, i.cols, i.rowStride, i.colStride};
+        }
+        appendToPlan(plan, it, true);
+        const uint64_t span = static_cast<uint64_t>((i.rows - 1) * i.rowStride + (i.cols - 1) * i.colStride + 1) * dtypeSize(i.from);
+        const uint64_t out = static_cast<uint64_t>(i.rows) * i.cols * dtypeSize(i.to);
+        srcOff += (i.srcOff + span + 255) / 256 * 256;
+        dstOff += (out + 255) / 256 * 256;
+        moved += it.srcBytes + out;
+      }
+      if (srcOff > bytes || dstOff > bytes) continue;
+      const double ms = timer.run(3, iters, [&] { launchPush(plan, nullptr, sms, nullptr, 0, nullptr, nullptr); });
+      std::printf("%-44s %10.1f us  %8.1f GB/s read+write\n", form.first, ms * 1e3, moved / (ms * 1e-3) / 1e9);
+    }
+  }
   if (want("mixed")) {
     // The 64-tensor message of the pipe benchmarks as ONE launch of the full kernel on one GPU:
     // dtype cycles fp32 / bf16 / int64, sizes log-uniform in [1 KiB, 16 MiB], every fourth tensor a

@@ -44,8 +44,9 @@ static __device__ __align__(256) unsigned char g_scratch[kCounterBytes];
 std::atomic<uint32_t> g_nextCounter{0};
 
 // Bound by memory: one warp per 8 KiB tile, 4 KiB of loads in flight per warp, 16 warps per SM; tiles meet
-// on 16-byte boundaries of the destination, so that only a range's own ends are ragged. (192 records of 1 MiB + 6 bytes packed densely, 201 MB: 508 us when ranges of
-// different alignment went byte by byte, 70 us now; the call 515 -> 76 us.)
+// on 16-byte boundaries of the destination, so that only a range's own ends are ragged. (192 records of 1 MiB + 6
+// bytes packed densely, 201 MB: 508 us when ranges of different alignment went byte by byte, 70 us now; the call
+// 515 -> 76 us.)
 // `counter` is one word of g_scratch; the host looks its address up.
 template <int N>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
