@@ -7,28 +7,34 @@
 //     entry whose source, destination and size are 16-byte multiples. The loads only ever read
 //     THIS GPU's memory; the stores may target a peer GPU's memory mapped over NVLink. No thread
 //     touches the bytes. Tile size and depth are run-time parameters (PushTuning).
-//   * The other warps handle what the bulk path cannot, one 8 KiB "warp tile" at a time and
+//   * The other warps handle what the bulk path cannot, one "warp tile" of up to 8 KiB at a time and
 //     without CTA-wide barriers: ragged heads and tails, relatively misaligned buffers, dtype
-//     conversion (fp32 <-> bf16/fp16), and 2-D strided sources, which a warp transposes through
+//     conversion (fp32 <-> bf16/fp16), views whose rows are contiguous (copied as the runs they
+//     are), and other 2-D strided sources, which a warp transposes through
 //     its private padded shared-memory tile so that both the strided reads and the packed writes
 //     are coalesced (32x32 elements; 64x64 moved as 32-bit words for 2-byte elements; 32 whole
 //     packed rows written as one contiguous run for matrices of at most 64 columns bound for
 //     another GPU). A warp makes one call per tensor for all of its tiles.
-//   * Tiles are dealt round-robin (bulk tile t to CTA t mod gridDim.x, warp tile t to warp
+//   * Large transposed matrices may move as "block tiles" instead, which eight warps share behind a
+//     barrier of their own: 128 bulk loads, sent for by as many threads, fill a stage of shared
+//     memory, and the warps write it out transposed.
+//   * Tiles are dealt round-robin (bulk and block tile t to CTA t mod gridDim.x, warp tile t to warp
 //     t mod #warps), so no scheduling state lives in global memory.
 //   * Completion: every CTA makes its writes visible system-wide, then arrives on a counter;
 //     the last CTA resets the counter and publishes the flag with a release store at system
 //     scope. The flag lives in the receiver's memory; its stream waits on it.
 //
-// A "light" instantiation (256 threads, no bulk pipeline, shared memory only when a tensor is
-// staged through it) serves messages without bulk work, where launch latency matters most.
+// A "light" instantiation (256 threads, no bulk copy engine, shared memory only when a tensor is
+// staged through it) serves messages without bulk work, where launch latency matters most. Both
+// come with the code for contiguous tensors only, for views moved by single warps too, and for all.
 //
 // Built with -DTPB_DEBUG_KERNELS the copy paths check every address against its table entry,
 // skip what lies outside and count it (boundsViolations()); nothing in here can trap.
 //
 // Every wait in here is bounded: a bulk load that does not complete within the limit makes the
-// CTA record kStatusBarrierTimeout, drain its own outstanding stores and fall through to the
-// completion protocol, so the kernel always terminates.
+// CTA record kStatusBarrierTimeout, drain its own outstanding stores (the block tiles: wait, again
+// within the limit, for their loads in flight) and fall through to the completion protocol, so the
+// kernel always terminates.
 #include "kernels/push.h"
 
 #include <cuda_bf16.h>
